@@ -296,6 +296,7 @@ void freeLayout(gf_engine *e) {
 }
 
 void freeNormEvents(gf_engine *e) {
+    dfree(e->d_ampc);
     for(auto &p : e->nscr)
         if(p)
             cudaFree(p);
@@ -584,6 +585,7 @@ GfArgs makeArgs(gf_engine *e) {
     a.nevt        = (const double *const *)e->d_nevt;
     a.nnorm       = e->d_nnorm;
     a.nscr        = (void *const *)e->d_nscr;
+    a.ampc        = e->d_ampc;
     a.gtoy        = 0;
     a.chunk       = e->chunk;
     a.nevt0       = e->toys.empty() ? 0 : e->toys[0].n;
@@ -817,7 +819,7 @@ int loadModule(gf_engine *e) {
        (rc = get(e->mod.val_n, "gf_val_n", true)))
         return rc;
     const bool hasAmp = e->tree.n_amp_nodes() > 0;
-    if((rc = get(e->mod.amp, "gf_amp", hasAmp)) || (rc = get(e->mod.ampn, "gf_ampn", hasAmp)) ||
+    if((rc = get(e->mod.ampc, "gf_ampc", e->plan.amp_terms > 0)) || (rc = get(e->mod.amp, "gf_amp", hasAmp)) || (rc = get(e->mod.ampn, "gf_ampn", hasAmp)) ||
        (rc = get(e->mod.gram, "gf_gram", hasAmp)))
         return rc;
     if((rc = get(e->mod.fcn_g, "gf_fcn_g", e->plan.fused)) || (rc = get(e->mod.fcn_n, "gf_fcn_n", e->plan.fused)))
@@ -1179,15 +1181,20 @@ int updateAmpCaches(gf_engine *e) {
         return GF_OK;
     fillRecords(e); // R copies of the parameters for the efficiency in the integral kernel
     int rc = e->amp_recompute ? GF_OK : ensureScratch(e);
+    const int nk = e->plan.amp_terms * e->plan.amp_term_k, ab = e->plan.amp_block;
+    if(rc == GF_OK && nk > 0 && !e->d_ampc)
+        rc = dalloc(e, e->d_ampc, (size_t)NT * nk);
     if(rc)
         return rc;
     GfArgs a      = makeArgs(e);
     cudaError_t r = cudaMemcpyAsync(e->d_P, e->h_P, e->pblock_bytes, cudaMemcpyHostToDevice, e->stream);
     if(r == cudaSuccess)
         r = cudaMemcpyAsync(e->d_dirty, e->h_dirty, sizeof(int) * NT, cudaMemcpyHostToDevice, e->stream);
+    if(r == cudaSuccess && anyData && nk > 0)
+        r = launch(e->mod.ampc, dim3((unsigned)e->plan.amp_terms, NT), dim3(32), 0, e->stream, a);
     if(r == cudaSuccess && anyData) {
-        const int64_t bx = std::min<int64_t>((maxpad + 255) / 256, (int64_t)std::max(1, e->sm_count) * 8);
-        r = launch(e->mod.amp, dim3((unsigned)bx, NT, (unsigned)NAN_), dim3(256), 0, e->stream, a);
+        const int64_t bx = std::min<int64_t>((maxpad + ab - 1) / ab, (int64_t)std::max(1, e->sm_count) * 16);
+        r = launch(e->mod.amp, dim3((unsigned)bx, NT, (unsigned)NAN_), dim3(ab), 0, e->stream, a);
     }
     if(r == cudaSuccess && anyData && !anyNorm)
         r = cudaStreamSynchronize(e->stream);
@@ -1200,7 +1207,7 @@ int updateAmpCaches(gf_engine *e) {
     int64_t maxpts = 1;
     for(int k = 0; k < NAN_; ++k)
         maxpts = std::max<int64_t>(maxpts, ampPoints(e, k));
-    const int64_t bn    = std::min<int64_t>((maxpts + 255) / 256, (int64_t)std::max(1, e->sm_count) * 8);
+    const int64_t bn    = std::min<int64_t>((maxpts + ab - 1) / ab, (int64_t)std::max(1, e->sm_count) * 16);
     const size_t gbytes = sizeof(double) * (size_t)NTILE * e->gram_blocks * PM2;
     for(int t = 0; t < NT && r == cudaSuccess; ++t) {
         if(!normDirty[t])
@@ -1209,7 +1216,7 @@ int updateAmpCaches(gf_engine *e) {
         // mode: one kernel that evaluates the amplitudes at every point and reduces them in place)
         a.gtoy = t;
         if(!e->amp_recompute)
-            r = launch(e->mod.ampn, dim3((unsigned)bn, 1, (unsigned)NAN_), dim3(256), 0, e->stream, a);
+            r = launch(e->mod.ampn, dim3((unsigned)bn, 1, (unsigned)NAN_), dim3(ab), 0, e->stream, a);
         GfToy &ty = e->toys[t];
         ty.amp_I.assign(NAN_, {});
         ty.amp_H.assign(NAN_, {});
@@ -1882,6 +1889,7 @@ int gf_set_num_toys(gf_engine *e, int n) {
         return gf_fail(e, GF_ERR_INVALID, "toy count must be >= 1");
     cudaSetDevice(e->device);
     freeLayout(e);
+    dfree(e->d_ampc);
     for(auto &t : e->toys)
         freeToy(t);
     e->n_toys = n;

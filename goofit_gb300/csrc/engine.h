@@ -52,6 +52,7 @@ struct GfArgs {
     unsigned bar_target;  // the arrival count at which this launch's grid barrier opens
     double *hpart;        // one-launch evaluation: per-chunk [components..., status] rows in page-locked memory
     const int *ksort;     // one-launch tabulated path: toy 0's bin offsets sorted by bin (null: read kcol)
+    const void *ampc;     // [toy][term][k] parameter-only constants of the Amp3Body resonances (gf_ampc)
     alignas(16) unsigned char rec[512];
     const void *p0[192];  // toy 0: observable columns, bin-offset columns, amplitude columns (one toy only)
 };
@@ -81,7 +82,7 @@ struct GfModule {
     cudaLibrary_t lib = nullptr;
     cudaKernel_t conv_g = nullptr, conv_n = nullptr, grid_g = nullptr, grid_n = nullptr;
     cudaKernel_t evt_g = nullptr, evt_n = nullptr, val_n = nullptr;
-    cudaKernel_t amp = nullptr, ampn = nullptr, gram = nullptr;
+    cudaKernel_t ampc = nullptr, amp = nullptr, ampn = nullptr, gram = nullptr;
     cudaKernel_t evt_gr = nullptr, gramr = nullptr; // amplitude recompute mode (gradient pass, integrals)
     cudaKernel_t fcn_g = nullptr, fcn_n = nullptr; // one toy: the whole evaluation in one cooperative launch
 };
@@ -150,6 +151,9 @@ struct gf_engine {
     double *d_gram = nullptr;    // integral partials [toy][tile][CTA][2 * pairs]
     double *h_gram = nullptr;
     int *d_dirty = nullptr, *h_dirty = nullptr;
+    // parameter-only constants of the Amp3Body resonances, 8 bytes each; kept with the amplitude caches they were
+    // built with, across layout rebuilds (freed with the tree or the toys)
+    unsigned long long *d_ampc = nullptr;
     int gram_blocks = 0;
     // Amp4Body normalisation events, one FP64 SoA [5][n] buffer per Amp4Body node (gf_set_norm_events)
     std::vector<double *> norm_buf;

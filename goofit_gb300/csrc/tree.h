@@ -215,6 +215,8 @@ struct KernelPlan {
     };
     std::vector<GramTile> gram_tiles;
     int gram_pairs_max = 0;                                 // most pairs in one tile
+    int amp_block = 128;                                    // threads per CTA of gf_amp and gf_ampn
+    int amp_terms = 0, amp_term_k = 0;                      // Amp3Body resonance terms, and constants of each (gf_ampc)
     std::vector<int64_t> dgrid_off;                         // per Amp3Body: offset of its bins in the bin list
     // the root's normalisation is applied on the host: the event pass returns sum -log P, sum -dP/P and the
     // count of events with P > 0 (out[2 + NG]); the host adds count * (-log N) and count * (-dN/N)
