@@ -282,10 +282,9 @@ void freeLayout(gf_engine *e) {
     dfree(e->d_dcols);
     dfree(e->d_dgrid);
     dfree(e->d_gram);
-    dfree(e->d_gtc_part);
-    dfree(e->d_gtc_out);
-    dfree(e->d_gtc_err);
-    e->gtc_part_n = e->gtc_out_n = 0;
+    dfree(e->d_gpart);
+    hfree(e->h_gout);
+    e->d_gout = nullptr;
     dfree(e->d_dirty);
     hfree(e->h_gram);
     hfree(e->h_dirty);
@@ -470,28 +469,12 @@ int buildLayout(gf_engine *e) {
     chk(dalloc(e, e->d_dgrid, std::max<size_t>(1, ngrid)));
     chk(dalloc(e, e->d_gram, (size_t)NT * std::max(1, NTILE) * e->gram_blocks * std::max(1, 2 * e->plan.gram_pairs_max)));
     chk(dalloc(e, e->d_dirty, NT));
-    // the integrals of the mixed-precision engine go through the tensor-core Gram kernel when every amplitude
-    // node has at most 32 complex columns (values and derivatives); GF_GRAM=cuda keeps the CUDA-core kernel
-    e->gram_tc = false;
-    if(e->precision == GF_MIXED && T.n_amp_nodes() > 0) {
-        const char *g = std::getenv("GF_GRAM");
-        e->gram_tc    = !(g && std::string(g) == "cuda");
-        size_t np = 0, no = 0;
-        for(int k = 0; k < T.n_amp_nodes(); ++k) {
-            const int nc = ampColumns(T, k);
-            if(gf_gram_tc_width(nc) == 0)
-                e->gram_tc = false;
-            np = std::max(np, gf_gram_tc_part_doubles(nc, std::max(1, e->sm_count)));
-            no = std::max(no, (size_t)4 * nc * nc);
-        }
-        if(e->gram_tc) {
-            chk(dalloc(e, e->d_gtc_part, np));
-            chk(dalloc(e, e->d_gtc_out, no));
-            chk(dalloc(e, e->d_gtc_err, 1));
-            e->gtc_part_n = np;
-            e->gtc_out_n  = no;
-            e->h_gtc.assign(no, 0.0);
-        }
+    if(e->plan.gram_tc) {
+        chk(dalloc(e, e->d_gpart, (size_t)e->gram_ctas * e->plan.gram_entries, false));
+        if(rc == GF_OK && (cudaHostAlloc((void **)&e->h_gout, sizeof(double) * (e->plan.gram_entries + 1),
+                                         cudaHostAllocMapped) != cudaSuccess ||
+                           cudaHostGetDevicePointer((void **)&e->d_gout, e->h_gout, 0) != cudaSuccess))
+            rc = gf_fail(e, GF_ERR_OOM, "cudaHostAlloc");
     }
     if(rc != GF_OK)
         return rc;
@@ -586,6 +569,12 @@ GfArgs makeArgs(gf_engine *e) {
     a.nnorm       = e->d_nnorm;
     a.nscr        = (void *const *)e->d_nscr;
     a.ampc        = e->d_ampc;
+    a.gpart       = e->d_gpart;
+    a.gram_ctas   = e->gram_ctas;
+    a.gram_ns     = e->gram_ns ? e->gram_ns : 2000000000ull;
+    a.gram_stall  = -1;
+    a.gout        = e->d_gout;
+    a.gerr        = e->d_gout ? reinterpret_cast<int *>(e->d_gout + e->plan.gram_entries) : nullptr;
     a.gtoy        = 0;
     a.chunk       = e->chunk;
     a.nevt0       = e->toys.empty() ? 0 : e->toys[0].n;
@@ -819,8 +808,9 @@ int loadModule(gf_engine *e) {
        (rc = get(e->mod.val_n, "gf_val_n", true)))
         return rc;
     const bool hasAmp = e->tree.n_amp_nodes() > 0;
-    if((rc = get(e->mod.ampc, "gf_ampc", e->plan.amp_terms > 0)) || (rc = get(e->mod.amp, "gf_amp", hasAmp)) || (rc = get(e->mod.ampn, "gf_ampn", hasAmp)) ||
-       (rc = get(e->mod.gram, "gf_gram", hasAmp)))
+    if((rc = get(e->mod.ampc, "gf_ampc", e->plan.amp_terms > 0)) || (rc = get(e->mod.amp, "gf_amp", hasAmp)) || (rc = get(e->mod.ampn, "gf_ampn", hasAmp && !e->plan.gram_tc)) ||
+       (rc = get(e->mod.gram, "gf_gram", hasAmp && !e->plan.gram_tc)) ||
+       (rc = get(e->mod.ampg, "gf_ampng", e->plan.gram_tc)) || (rc = get(e->mod.ampg_sum, "gf_ampng_sum", e->plan.gram_tc)))
         return rc;
     if((rc = get(e->mod.fcn_g, "gf_fcn_g", e->plan.fused)) || (rc = get(e->mod.fcn_n, "gf_fcn_n", e->plan.fused)))
         return rc;
@@ -839,7 +829,7 @@ int loadModule(gf_engine *e) {
        (rc = smem(e->mod.evt_g, e->plan.evt_smem_grad)) || (rc = smem(e->mod.evt_n, e->plan.evt_smem_nograd)) ||
        (rc = smem(e->mod.evt_gr, e->plan.evt_smem_gr)) ||
        (rc = smem(e->mod.val_n, e->plan.evt_smem_nograd)) || (rc = smem(e->mod.fcn_g, e->plan.fused_smem[1])) ||
-       (rc = smem(e->mod.fcn_n, e->plan.fused_smem[0])))
+       (rc = smem(e->mod.fcn_n, e->plan.fused_smem[0])) || (rc = smem(e->mod.ampg, e->plan.gram_smem)))
         return rc;
     const size_t maxSmem = 227 * 1024;
     if(e->plan.conv_smem_grad > maxSmem || e->plan.evt_smem_grad > maxSmem)
@@ -1180,7 +1170,8 @@ int updateAmpCaches(gf_engine *e) {
     if(!anyData && !anyNorm)
         return GF_OK;
     fillRecords(e); // R copies of the parameters for the efficiency in the integral kernel
-    int rc = e->amp_recompute ? GF_OK : ensureScratch(e);
+    const bool tc = e->plan.gram_tc && !e->amp_recompute;
+    int rc = e->amp_recompute || tc ? GF_OK : ensureScratch(e);
     const int nk = e->plan.amp_terms * e->plan.amp_term_k, ab = e->plan.amp_block;
     if(rc == GF_OK && nk > 0 && !e->d_ampc)
         rc = dalloc(e, e->d_ampc, (size_t)NT * nk);
@@ -1215,40 +1206,30 @@ int updateAmpCaches(gf_engine *e) {
         // the normalisation points of this toy: amplitudes (and derivatives), then their reduction (recompute
         // mode: one kernel that evaluates the amplitudes at every point and reduces them in place)
         a.gtoy = t;
-        if(!e->amp_recompute)
+        if(!e->amp_recompute && !tc)
             r = launch(e->mod.ampn, dim3((unsigned)bn, 1, (unsigned)NAN_), dim3(ab), 0, e->stream, a);
         GfToy &ty = e->toys[t];
         ty.amp_I.assign(NAN_, {});
         ty.amp_H.assign(NAN_, {});
-        if(e->gram_tc && !e->amp_recompute) {
-            // tensor cores: the real Gram matrix G of each node's columns, then I and H from its blocks
-            for(int k = 0; k < NAN_ && r == cudaSuccess; ++k) {
-                const int n = T.amp_count(k), nc = ampColumns(T, k), m = 2 * nc;
-                const int64_t npts = ampPoints(e, k), nst = ampStride(e, k);
-                const float2 *sc   = reinterpret_cast<const float2 *>(e->nscr[k]);
-                const float *eff   = k < (int)T.amp3s.size() ? reinterpret_cast<const float *>(sc + (size_t)nc * nst) : nullptr;
-                int herr           = 0;
-                r = cudaMemsetAsync(e->d_gtc_err, 0, sizeof(int), e->stream);
-                // GF_GRAM_TEST_STALL_STAGE (tests of the failure path): the wait for that stage runs out
-                const char *stall = std::getenv("GF_GRAM_TEST_STALL_STAGE");
-                if(r == cudaSuccess)
-                    r = gf_gram_tc_launch(sc, npts, nst, nc, eff, std::max(1, e->sm_count), e->d_gtc_part,
-                                          e->d_gtc_out, e->d_gtc_err, e->stream,
-                                          e->gram_w >= gf_gram_tc_width(nc) ? e->gram_w : 0, e->gram_ns,
-                                          stall && *stall ? std::atoi(stall) : -1);
-                if(r == cudaSuccess)
-                    r = cudaMemcpyAsync(e->h_gtc.data(), e->d_gtc_out, sizeof(double) * (size_t)m * m,
-                                        cudaMemcpyDeviceToHost, e->stream);
-                if(r == cudaSuccess)
-                    r = cudaMemcpyAsync(&herr, e->d_gtc_err, sizeof(int), cudaMemcpyDeviceToHost, e->stream);
-                if(r == cudaSuccess)
-                    r = cudaStreamSynchronize(e->stream);
-                if(r != cudaSuccess)
-                    break;
-                if(herr)
-                    return gf_fail(e, GF_ERR_CUDA, "tensor-core Gram kernel: a bounded wait ran out");
-                const double *G = e->h_gtc.data();
-                // X_a conj(X_b) summed: Re = G(re a, re b) + G(im a, im b), Im = G(im a, re b) - G(re a, im b)
+        if(tc) {
+            int *err = reinterpret_cast<int *>(e->h_gout + e->plan.gram_entries);
+            *err     = 0;
+            // GF_GRAM_TEST_STALL_STAGE (tests of the failure path): the wait for that tile runs out
+            const char *stall = std::getenv("GF_GRAM_TEST_STALL_STAGE");
+            a.gram_stall      = stall && *stall ? std::atoi(stall) : -1;
+            r = launch(e->mod.ampg, dim3((unsigned)e->gram_ctas, 1, (unsigned)NAN_), dim3(ab), e->plan.gram_smem, e->stream, a);
+            if(r == cudaSuccess)
+                r = launch(e->mod.ampg_sum, dim3((unsigned)e->plan.gram_entries), dim3(128), 0, e->stream, a);
+            if(r == cudaSuccess)
+                r = cudaStreamSynchronize(e->stream);
+            if(r != cudaSuccess)
+                break;
+            if(*reinterpret_cast<volatile int *>(err))
+                return gf_fail(e, GF_ERR_CUDA, "tensor-core integrals: a bounded wait ran out");
+            for(int k = 0; k < NAN_; ++k) {
+                const int n = T.amp_count(k), nc = ampColumns(T, k), m = 2 * n;
+                const double *G = e->h_gout + e->plan.gram_off[k];
+                // X_u conj(X_v) summed: Re = G(re u, re v) + G(im u, im v), Im = G(im u, re v) - G(re u, im v)
                 auto ent = [&](int u, int v, double &re, double &im) {
                     re = G[(size_t)(2 * u) * m + 2 * v] + G[(size_t)(2 * u + 1) * m + 2 * v + 1];
                     im = G[(size_t)(2 * u + 1) * m + 2 * v] - G[(size_t)(2 * u) * m + 2 * v + 1];
@@ -1268,11 +1249,9 @@ int updateAmpCaches(gf_engine *e) {
                 for(int d = 0; d < nc - n; ++d)
                     for(int b = 0; b < n; ++b)
                         ent(n + d, b, H[2 * (d * n + b)], H[2 * (d * n + b) + 1]);
-                ty.amp_I[k] = I;
-                ty.amp_H[k] = H;
+                ty.amp_I[k] = std::move(I);
+                ty.amp_H[k] = std::move(H);
             }
-            if(r != cudaSuccess)
-                break;
             ty.amp_params = snap[t];
             ty.norm_valid = true;
             continue;
@@ -1854,6 +1833,26 @@ static int compileTree(gf_engine *e) {
             occ = 0;
         }
         e->evt_ctas_per_sm = std::min(8, std::max(1, occ));
+    }
+    // the tensor-core integrals: persistent CTAs, as many as registers, shared memory and tensor memory keep resident
+    // (the runtime's occupancy query answers one for a kernel that allocates tensor memory)
+    e->gram_ctas = 0;
+    if(e->plan.gram_tc) {
+        cudaFuncAttributes fa{};
+        int smemSM = 0, regsSM = 0, reserved = 0;
+        cudaError_t r = cudaFuncGetAttributes(&fa, (const void *)e->mod.ampg);
+        if(r == cudaSuccess)
+            r = cudaDeviceGetAttribute(&smemSM, cudaDevAttrMaxSharedMemoryPerMultiprocessor, e->device);
+        if(r == cudaSuccess)
+            r = cudaDeviceGetAttribute(&regsSM, cudaDevAttrMaxRegistersPerMultiprocessor, e->device);
+        if(r == cudaSuccess)
+            r = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, e->device);
+        if(r != cudaSuccess)
+            return gf_cuda_check(e, r, "tensor-core integral kernel attributes");
+        const int regs = (std::max(1, fa.numRegs) + 7) / 8 * 8 * e->plan.amp_block;
+        const int smem = (int)(e->plan.gram_smem + fa.sharedSizeBytes) + reserved;
+        const int occ  = std::min(512 / e->plan.gram_tmem, std::min(regsSM / regs, smemSM / smem));
+        e->gram_ctas   = std::max(1, occ) * std::max(1, e->sm_count);
     }
     // the one-launch kernel's grid: every CTA resident (a cooperative launch), at most as many per SM as the
     // event kernel's chunk layout assumes
@@ -2437,7 +2436,6 @@ int applyShapes(gf_engine *e, const gf::Shapes &sh, const std::vector<double> &P
 
 struct TunedShapes {
     gf::Shapes sh;
-    int gram_w = 0;
 };
 
 } // namespace
@@ -2466,7 +2464,6 @@ int gf_tune_shapes(gf_engine *e) {
         std::lock_guard<std::mutex> lk(mu);
         auto it = cache.find(key);
         if(it != cache.end()) {
-            e->gram_w = it->second.gram_w;
             if(it->second.sh.conv_kp == e->plan.conv_kp && it->second.sh.grid_bpb == e->plan.grid_bins_per_block)
                 return GF_OK;
             return applyShapes(e, it->second.sh, P, act);
@@ -2522,43 +2519,9 @@ int gf_tune_shapes(gf_engine *e) {
        e->plan.conv_kp != best.conv_kp || e->plan.grid_bins_per_block != best.grid_bpb)
         if((rc = applyShapes(e, best, P, act)))
             return rc;
-    // tensor-core Gram slice width: the integral rebuild timed at every width the widest node allows
-    int bestW = 0;
-    if(e->gram_tc && !e->amp_recompute && T.n_amp_nodes() > 0) {
-        int wmin = 16;
-        for(int k = 0; k < T.n_amp_nodes(); ++k)
-            wmin = std::max(wmin, gf_gram_tc_width(ampColumns(T, k)));
-        double bestG = 1e30;
-        for(int w : {16, 32, 64}) {
-            if(w < wmin)
-                continue;
-            e->gram_w = w;
-            double mn = 1e30;
-            for(int it = 0; it < 4; ++it) {
-                for(auto &ty : e->toys)
-                    ty.norm_valid = false;
-                if(flush)
-                    cudaMemsetAsync(flush, it & 0xff, flushBytes, e->stream);
-                cudaStreamSynchronize(e->stream);
-                const auto t0 = std::chrono::steady_clock::now();
-                if((rc = updateAmpCaches(e)))
-                    return rc;
-                const double ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-                if(it > 0)
-                    mn = std::min(mn, ms);
-            }
-            if(mn < bestG) {
-                bestG = mn;
-                bestW = w;
-            }
-        }
-        e->gram_w = bestW;
-        for(auto &ty : e->toys)
-            ty.norm_valid = false;
-    }
     {
         std::lock_guard<std::mutex> lk(mu);
-        cache[key] = TunedShapes{best, bestW};
+        cache[key] = TunedShapes{best};
     }
     return GF_OK;
 }
@@ -2570,12 +2533,8 @@ int gf_get_shapes(const gf_engine *e, int32_t *conv_kp, int32_t *grid_bpb, int32
         *conv_kp = e->plan.conv_kp;
     if(grid_bpb)
         *grid_bpb = e->plan.grid_bins_per_block;
-    if(gram_w) {
-        int w = 0;
-        for(int k = 0; k < e->tree.n_amp_nodes(); ++k)
-            w = std::max(w, gf_gram_tc_width(ampColumns(e->tree, k)));
-        *gram_w = e->gram_tc ? std::max(e->gram_w, w) : 0;
-    }
+    if(gram_w)
+        *gram_w = e->plan.gram_w;
     return GF_OK;
 }
 

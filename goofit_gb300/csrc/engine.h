@@ -53,6 +53,12 @@ struct GfArgs {
     double *hpart;        // one-launch evaluation: per-chunk [components..., status] rows in page-locked memory
     const int *ksort;     // one-launch tabulated path: toy 0's bin offsets sorted by bin (null: read kcol)
     const void *ampc;     // [toy][term][k] parameter-only constants of the Amp3Body resonances (gf_ampc)
+    double *gpart;        // tensor-core integrals: [entry][CTA] partials of gram_ctas CTAs, their sums in page-locked
+    double *gout;         // memory, the error word and the longest wait for a tile's MMAs
+    int *gerr;
+    unsigned long long gram_ns;
+    int gram_ctas;
+    int gram_stall;       // test of the failure path: the tile whose wait runs out (-1: none)
     alignas(16) unsigned char rec[512];
     const void *p0[192];  // toy 0: observable columns, bin-offset columns, amplitude columns (one toy only)
 };
@@ -83,6 +89,7 @@ struct GfModule {
     cudaKernel_t conv_g = nullptr, conv_n = nullptr, grid_g = nullptr, grid_n = nullptr;
     cudaKernel_t evt_g = nullptr, evt_n = nullptr, val_n = nullptr;
     cudaKernel_t ampc = nullptr, amp = nullptr, ampn = nullptr, gram = nullptr;
+    cudaKernel_t ampg = nullptr, ampg_sum = nullptr; // tensor-core integrals, in place of ampn and gram
     cudaKernel_t evt_gr = nullptr, gramr = nullptr; // amplitude recompute mode (gradient pass, integrals)
     cudaKernel_t fcn_g = nullptr, fcn_n = nullptr; // one toy: the whole evaluation in one cooperative launch
 };
@@ -116,10 +123,8 @@ struct gf_engine {
     bool amp_recompute   = false;
     bool amp_decided     = false;
 
-    // launch shapes (gf_tune_shapes): the generator's table k-tiles and grid bins per CTA, and the tensor-core
-    // Gram kernel's slice width (0: the defaults)
+    // launch shapes (gf_tune_shapes): the generator's table k-tiles and grid bins per CTA (0: the defaults)
     gf::Shapes shapes;
-    int gram_w = 0;
 
     int fit_metric = GF_FIT_UNBINNED_NLL;
     int n_toys = 1;
@@ -160,14 +165,13 @@ struct gf_engine {
     std::vector<int64_t> norm_n;
     double **d_nevt = nullptr;
     long long *d_nnorm = nullptr;
-    // normalisation-point columns per amplitude node (values, derivatives, efficiency) of one toy at a time
-    // tensor-core Gram (mixed precision): per-CTA FP64 partials, the summed real Gram matrix, a status word
-    bool gram_tc         = false;
-    double *d_gtc_part   = nullptr;
-    double *d_gtc_out    = nullptr;
-    int *d_gtc_err       = nullptr;
-    size_t gtc_part_n    = 0, gtc_out_n = 0;
-    std::vector<double> h_gtc;
+    // tensor-core integrals (mixed precision, gf_ampng): CTAs, their FP64 partials, and in one mapped page-locked block
+    // the summed entries followed by the error word
+    int gram_ctas      = 0;
+    double *d_gpart    = nullptr;
+    double *h_gout = nullptr, *d_gout = nullptr;
+    // normalisation-point columns per amplitude node (values, derivatives, efficiency) of one toy at a time, where
+    // gf_ampn and gf_gram form the integrals
     std::vector<void *> nscr;
     std::vector<size_t> nscr_bytes;
     void **d_nscr = nullptr;
@@ -204,7 +208,7 @@ struct gf_engine {
     int fcn_grid          = 0;
     unsigned *d_gbar      = nullptr;
     unsigned long long bar_ns = 1000000000ull;
-    unsigned long long gram_ns = 0; // per-stage wait limit of the tensor-core Gram kernel (0: its 2 s default)
+    unsigned long long gram_ns = 0; // wait limit of gf_ampng for a tile's MMAs (0: 2 s)
     unsigned bar_epoch        = 0; // one-launch evaluations run since the barrier words were cleared
     bool fused_graph_ok   = true; // false: the cooperative launch is not captured into a graph here
     // captured one-launch graphs [nograd, grad]: the source graph, its kernel node and that node's launch
@@ -220,18 +224,5 @@ struct gf_engine {
 // helpers shared between translation units
 int gf_fail(gf_engine *e, int code, const std::string &msg);
 
-// tensor-core Gram matrix of ncol complex FP32 columns (gram_tc.cu): real columns per slice (16, 32 or 64),
-// 0 when 2 ncol > 64
-int gf_gram_tc_width(int ncol);
-size_t gf_gram_tc_part_doubles(int ncol, int grid);
-// G (2 ncol x 2 ncol, FP64) = sum_{p < npts} x_r(p) eff(p) x_s(p) of the columns sc[c * nst + p] (nst a
-// multiple of 4, sc and eff 16-byte aligned) into out; part holds gf_gram_tc_part_doubles(ncol, sm_count)
-// doubles; *err gets bit 0 when a bounded wait ran out; width: real columns per slice (16, 32 or 64, at least
-// gf_gram_tc_width(ncol)), 0 for the narrowest; wait_ns: the limit of each per-stage mbarrier wait (0: 2 s; the
-// wait for the last committed MMAs before the tensor memory is freed is always 2 s); stall >= 0: a test of the
-// failure path, in which the wait for stage `stall` also waits on a barrier that never completes
-cudaError_t gf_gram_tc_launch(const float2 *sc, long long npts, long long nst, int ncol, const float *eff,
-                              int sm_count, double *part, double *out, int *err, cudaStream_t s, int width = 0,
-                              unsigned long long wait_ns = 0, int stall = -1);
 int gf_cuda_check(gf_engine *e, cudaError_t r, const char *what);
 int gf_run(gf_engine *e, bool grad, int metric_values_toy, int metric);

@@ -214,6 +214,12 @@ struct KernelPlan {
         int amp, p0, p1; // node index in Tree::amp3s, pair range
     };
     std::vector<GramTile> gram_tiles;
+    // tensor-core integrals (gf_ampng, mixed engine): dynamic shared memory, the widest slice, every node's first entry
+    // of G (2C x 2n) and their number.  GF_GRAM=cuda and nodes of more than 32 complex columns take gf_ampn and gf_gram
+    bool gram_tc     = false;
+    size_t gram_smem = 0;
+    int gram_w = 0, gram_tmem = 32, gram_entries = 0; // and tensor-memory columns of a CTA
+    std::vector<int> gram_off;
     int gram_pairs_max = 0;                                 // most pairs in one tile
     int amp_block = 128;                                    // threads per CTA of gf_amp and gf_ampn
     int amp_terms = 0, amp_term_k = 0;                      // Amp3Body resonance terms, and constants of each (gf_ampc)

@@ -235,7 +235,7 @@ class Engine:
         self._check(self._L.gf_set_wait_limit(self._h, int(ns)))
 
     def set_gram_wait_limit(self, ns: int) -> None:
-        """Longest wait of each pipeline stage of the tensor-core Gram kernel (ns; 0: the default 2 s)."""
+        """Longest wait for a tile's products in the tensor-core integral kernel (ns; 0: the default 2 s)."""
         self._check(self._L.gf_set_gram_wait_limit(self._h, int(ns)))
 
     def set_amp_mode(self, mode: str, budget_bytes: int = 0) -> None:
@@ -255,7 +255,7 @@ class Engine:
         return int(self._L.gf_amp_store_bytes(self._h))
 
     def tune_shapes(self) -> dict:
-        """Runs the launch-shape autotuner (table k-tiles, grid bins per CTA, Gram slice width) on the uploaded
+        """Runs the launch-shape autotuner (table k-tiles, grid bins per CTA) on the uploaded
         events and returns the shapes in use."""
         self._check(self._L.gf_tune_shapes(self._h))
         return self.shapes()

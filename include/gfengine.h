@@ -208,8 +208,8 @@ int64_t gf_event_chunk(const gf_engine *eng);
  * A wait that runs out stops the launch, the call returns GF_ERR_TIMEOUT and the engine stays usable.
  * No counterpart in the reference (its Thrust reductions have no device-side waits). */
 int gf_set_wait_limit(gf_engine *eng, uint64_t ns);
-/* Longest wait, in nanoseconds of the GPU's global timer, of each pipeline-stage mbarrier wait of the mixed
- * engine's tensor-core Gram kernel (the normalisation integrals of Amp3Body / Amp4Body); ns = 0 restores the
+/* Longest wait, in nanoseconds of the GPU's global timer, of each tile's mbarrier wait of the mixed engine's
+ * tensor-core integral kernel (the normalisation integrals of Amp3Body / Amp4Body); ns = 0 restores the
  * default of 2 s.  The kernel's wait for its last committed MMAs before it frees its tensor memory always keeps
  * the 2 s limit.  A wait that runs out makes the integral rebuild return GF_ERR_CUDA; the engine stays usable
  * and rebuilds the integrals at the next evaluation.  No counterpart in the reference (its integrals are
@@ -236,12 +236,12 @@ int64_t gf_amp_store_bytes(const gf_engine *eng);
 /* Launch-shape autotuner (the counterpart of the reference's grain-size sweep, scripts/find_optimal.py): times
    one gradient evaluation of every toy (device time, L2 flushed) for each candidate and keeps the fastest.
    Candidates: the table kernel's k-tiles per staged model and resolution (1, 2, 4, 8; batches of toys with a
-   convolution), the numeric-grid bins per CTA (128 ... 2048; grids not folded into a table), then the
-   tensor-core Gram kernel's slice width (16, 32, 64 real columns; the integral rebuild timed).  Each table or
-   grid candidate recompiles the tree.  Needs uploaded events; results are remembered for the process, keyed by
+   convolution) and the numeric-grid bins per CTA (128 ... 2048; grids not folded into a table).  Each
+   candidate recompiles the tree.  Needs uploaded events; results are remembered for the process, keyed by
    tree, precision, toy count and events. */
 int gf_tune_shapes(gf_engine *eng);
-/* The shapes in use: table k-tiles, grid bins per CTA, Gram slice width (0: no tensor-core Gram). */
+/* The shapes in use: table k-tiles, grid bins per CTA, and the real columns per slice of the tensor-core integrals
+   (32 or 64 by the widest amplitude node; 0: none). */
 int gf_get_shapes(const gf_engine *eng, int32_t *conv_kp, int32_t *grid_bpb, int32_t *gram_w);
 
 /* ---- minimiser (Minuit2 MnMigrad surface, src/goofit/FitManagerMinuit2.cpp:31-119) ---- */
