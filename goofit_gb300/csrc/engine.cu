@@ -729,7 +729,7 @@ cudaError_t enqueueEval(gf_engine *e, bool grad) {
             cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
             if(r == cudaSuccess && cudaStreamIsCapturing(e->stream, &cs) == cudaSuccess &&
                cs == cudaStreamCaptureStatusNone)
-                ++e->bar_epoch;
+                e->bar_epoch += (unsigned)e->plan.fused_barriers[grad ? 1 : 0];
         }
         if(r == cudaSuccess)
             r = recordEvent(e, e->ev[3]);
@@ -1584,7 +1584,7 @@ int gf_run(gf_engine *e, bool grad, int, int) {
                 } else {
                     r = cudaGraphLaunch(ge, e->stream);
                     if(r == cudaSuccess)
-                        ++e->bar_epoch;
+                        e->bar_epoch += (unsigned)e->plan.fused_barriers[grad ? 1 : 0];
                 }
             } else
                 r = cudaGraphLaunch(ge, e->stream);

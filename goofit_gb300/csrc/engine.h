@@ -49,7 +49,7 @@ struct GfArgs {
     int rec_n;            // one-launch evaluation: the toy's record (rec_n R values) passed by value in rec
     int stage_off;        // one-launch evaluation: shared-memory offset and room (bytes) of the staged events
     unsigned stage_cap;
-    unsigned bar_target;  // the arrival count at which this launch's grid barrier opens
+    unsigned bar_target;  // the arrival count at which this launch's first grid barrier opens
     double *hpart;        // one-launch evaluation: per-chunk [components..., status] rows in page-locked memory
     const int *ksort;     // one-launch tabulated path: toy 0's bin offsets sorted by bin (null: read kcol)
     const void *ampc;     // [toy][term][k] parameter-only constants of the Amp3Body resonances (gf_ampc)
@@ -209,7 +209,7 @@ struct gf_engine {
     unsigned *d_gbar      = nullptr;
     unsigned long long bar_ns = 1000000000ull;
     unsigned long long gram_ns = 0; // wait limit of gf_ampng for a tile's MMAs (0: 2 s)
-    unsigned bar_epoch        = 0; // one-launch evaluations run since the barrier words were cleared
+    unsigned bar_epoch        = 0; // grid barriers of one-launch evaluations since the barrier words were cleared
     bool fused_graph_ok   = true; // false: the cooperative launch is not captured into a graph here
     // captured one-launch graphs [nograd, grad]: the source graph, its kernel node and that node's launch
     // parameters, whose arguments (the toy's record by value) are replaced before every graph launch

@@ -233,6 +233,7 @@ struct KernelPlan {
     size_t fused_smem[2] = {0, 0};      // dynamic shared memory, staged events included
     size_t fused_stage_off[2] = {0, 0}; // where the staged events start (after the tables' working space)
     size_t fused_stage_cap[2] = {0, 0}; // and the bytes of them that fit
+    int fused_barriers[2] = {0, 0};     // grid barriers of a launch
     int fused_row[2] = {0, 0};          // doubles per chunk row it writes to host memory (components, status)
     NormLayout nl;
 };
