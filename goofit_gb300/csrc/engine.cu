@@ -401,6 +401,14 @@ int buildLayout(gf_engine *e) {
     for(int t = 0; t < NT; ++t)
         if(!e->toys[t].loaded)
             return gf_fail(e, GF_ERR_STATE, "toy " + std::to_string(t) + " has no events");
+    // one-launch evaluation: every resident CTA, but one per SM where the FP64 engine tabulates the event terms and one
+    // CTA's share of the events fits its shared memory: every CTA repeats the table fold, its terms and its reductions
+    // in FP64, which the SM's CTAs share (1e5 events: 41 us with one, 45 us with two)
+    e->fcn_grid = e->fcn_per_sm * e->sm_count;
+    if(e->precision == GF_FP64 && e->plan.fused_tab && e->fcn_per_sm > 1 &&
+       (e->toys[0].n / e->sm_count + 2 * 256) * (int64_t)sizeof(int) <=
+           (int64_t)std::min(e->plan.fused_stage_cap[0], e->plan.fused_stage_cap[1]))
+        e->fcn_grid = e->sm_count;
     // chunk size: one chunk per resident event CTA (SMs x the event kernel's occupancy), so that a single
     // wave covers every SM with equal work; a multiple of 256 events (a warp's pass at 8 events per thread)
     if(!e->chunk_fixed) {
@@ -442,7 +450,7 @@ int buildLayout(gf_engine *e) {
     int64_t ctab = std::max(e->plan.ctab_per_toy_grad, e->plan.ctab_per_toy_nograd);
     {
         void *p = nullptr;
-        size_t bytes = (size_t)std::max<int64_t>(1, NT * ctab) * rsize(e);
+        size_t bytes = (size_t)std::max<int64_t>({1, NT * ctab, e->plan.ctab_elements}) * rsize(e);
         if(cudaMalloc(&p, bytes) != cudaSuccess)
             chk(gf_fail(e, GF_ERR_OOM, "cudaMalloc conv tables"));
         else
@@ -1856,7 +1864,7 @@ static int compileTree(gf_engine *e) {
     }
     // the one-launch kernel's grid: every CTA resident (a cooperative launch), at most as many per SM as the
     // event kernel's chunk layout assumes
-    e->fcn_grid = 0;
+    e->fcn_per_sm = e->fcn_grid = 0;
     if(e->plan.fused && e->mod.fcn_g && e->mod.fcn_n) {
         int o1 = 0, o0 = 0;
         if(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o1, (const void *)e->mod.fcn_g, e->block,
@@ -1867,7 +1875,8 @@ static int compileTree(gf_engine *e) {
             o1 = o0 = 0;
         }
         const int per = std::min(std::min(o1, o0), e->evt_ctas_per_sm);
-        e->fcn_grid   = per > 0 ? per * e->sm_count : 0;
+        e->fcn_per_sm = per > 0 ? per : 0;
+        e->fcn_grid   = e->fcn_per_sm * e->sm_count;
     }
     return GF_OK;
 }

@@ -205,7 +205,7 @@ struct gf_engine {
     bool use_fused        = true;
     bool use_stage        = true; // GF_STAGE=0: the one-launch kernel reads events from global memory
     bool use_ksort        = true; // GF_KSORT=0: its tabulated event pass reads the offsets in upload order
-    int fcn_grid          = 0;
+    int fcn_per_sm = 0, fcn_grid = 0; // CTAs that stay resident on an SM; CTAs of a launch
     unsigned *d_gbar      = nullptr;
     unsigned long long bar_ns = 1000000000ull;
     unsigned long long gram_ns = 0; // wait limit of gf_ampng for a tile's MMAs (0: 2 s)

@@ -203,6 +203,7 @@ struct KernelPlan {
     std::vector<char> num_folded; // per numeric node
     bool grid_needs_conv = false; // an unfolded numeric node reads a convolution table
     int64_t ctab_per_toy_grad = 0, ctab_per_toy_nograd = 0; // table elements per toy
+    int64_t ctab_elements = 0; // of one toy's tables and what is staged behind them (one toy, FP64)
     std::vector<int64_t> ctab_off_grad, ctab_off_nograd;    // per conv
     // mixed precision, one toy: the low parts of conv 0's values (the table's value column holds the high parts
     // of unevaluated FP32 pairs), at this element offset of the toy's table block; -1 when not kept
