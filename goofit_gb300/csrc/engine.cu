@@ -960,6 +960,10 @@ void fillRecordsT(gf_engine *e) {
             Pq[j] = (double)r[j];
         }
         const double *P = Pq.data();
+        auto split      = [](R *q, double v) {
+            q[0] = (R)v;
+            q[1] = (R)(v - (double)q[0]);
+        };
         for(auto &an : nl.analytic) {
             const gf::TNode &nd = T.nodes[an.node];
             if(an.kind == gf::NK_AMP3 || an.kind == gf::NK_AMP4) {
@@ -970,7 +974,7 @@ void fillRecordsT(gf_engine *e) {
                 r[an.slotN]     = (R)N;
                 r[an.slotNL]    = (R)(N - (double)(R)N);
                 for(size_t k = 0; k < an.dN.size(); ++k)
-                    r[an.dN[k].second] = (R)(-N * N * f * dQ[k]);
+                    split(r + an.dN[k].second, -N * N * f * dQ[k]);
                 if(an.node == 0) {
                     e->root_N[t] = N;
                     for(size_t k = 0; k < an.dN.size(); ++k)
@@ -1008,7 +1012,7 @@ void fillRecordsT(gf_engine *e) {
             r[an.slotN]    = (R)N;
             r[an.slotNL]   = (R)(N - (double)(R)N);
             for(auto &d : an.dN)
-                r[d.second] = (R)(-N * N * dI);
+                split(r + d.second, -N * N * dI);
             if(an.node == 0) {
                 e->root_N[t] = N;
                 for(auto &d : an.dN)
