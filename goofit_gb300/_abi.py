@@ -137,6 +137,7 @@ SIGNATURES = [
     ("gf_set_params", C.c_int, [_vp, C.c_int, _f64p, C.c_int]),
     ("gf_nll", C.c_int, [_vp, C.c_int, _f64p]),
     ("gf_nll_grad", C.c_int, [_vp, C.c_int, _f64p, _f64p]),
+    ("gf_nll_at", C.c_int, [_vp, C.c_int, _vp, C.c_int, _vp, _vp]),
     ("gf_nll_batch", C.c_int, [_vp, C.c_int, _f64p, _i32p, _f64p, _f64p]),
     ("gf_num_grad", C.c_int, [_vp]),
     ("gf_num_params", C.c_int, [_vp]),

@@ -2128,6 +2128,12 @@ int gf_nll(gf_engine *e, int toy, double *nll) { return evalOne(e, toy, false, n
 
 int gf_nll_grad(gf_engine *e, int toy, double *nll, double *grad) { return evalOne(e, toy, true, nll, grad); }
 
+int gf_nll_at(gf_engine *e, int toy, const double *p, int n, double *nll, double *grad) {
+    if(int rc = gf_set_params(e, toy, p, n))
+        return rc;
+    return evalOne(e, toy, grad != nullptr, nll, grad);
+}
+
 int gf_num_grad(const gf_engine *e) { return e && e->has_tree ? e->tree.NG : 0; }
 int gf_num_params(const gf_engine *e) { return e && e->has_tree ? e->tree.n_params : 0; }
 int gf_num_toys(const gf_engine *e) { return e ? e->n_toys : 0; }

@@ -135,6 +135,12 @@ class Engine:
         buf = (C.c_int32 * max(1, self.n_grad))()
         self._L.gf_grad_params(self._h, buf, self.n_grad)
         self.grad_params = [buf[i] for i in range(self.n_grad)]
+        # parameters in, value and gradient out of the calls at a point: one array whose addresses are passed as
+        # numbers (two calls with ctypes pointers to fresh arrays took 7 us of a 19 us call)
+        n = self.n_params
+        self._io = np.zeros(n + 1 + self.n_grad)
+        self._in, self._out = self._io[:n], self._io[n + 1:]
+        self._at = self._io.ctypes.data
         self.n_toys = 1
         self._n_events = {}
 
@@ -159,8 +165,23 @@ class Engine:
         arr, p = A.f64(params)
         self._check(self._L.gf_set_params(self._h, toy, p, len(arr)))
 
+    def _eval_at(self, params, toy: int, grad: bool) -> bool:
+        """Evaluates at params into self._io; False (nothing done) when params is not one value per parameter."""
+        a = np.asarray(params, dtype=np.float64)
+        n = self.n_params
+        if n == 0 or a.shape != (n,):
+            return False
+        self._in[:] = a
+        at = self._at
+        rc = self._L.gf_nll_at(self._h, toy, at, n, at + 8 * n, at + 8 * n + 8 if grad else None)
+        if rc:
+            self._check(rc)
+        return True
+
     def nll(self, params=None, toy: int = 0) -> float:
         if params is not None:
+            if self._eval_at(params, toy, False):
+                return self._io.item(self.n_params)
             self.set_params(params, toy)
         out = C.c_double()
         self._check(self._L.gf_nll(self._h, toy, C.byref(out)))
@@ -168,6 +189,8 @@ class Engine:
 
     def nll_grad(self, params=None, toy: int = 0) -> tuple[float, np.ndarray]:
         if params is not None:
+            if self.n_grad and self._eval_at(params, toy, True):
+                return self._io.item(self.n_params), self._out.copy()
             self.set_params(params, toy)
         out = C.c_double()
         g = np.zeros(max(1, self.n_grad))

@@ -175,6 +175,8 @@ int gf_set_params(gf_engine *eng, int toy, const double *params, int n_params);
 int gf_nll(gf_engine *eng, int toy, double *nll);
 /* grad has one entry per parameter whose grad_mask is set, in parameter order */
 int gf_nll_grad(gf_engine *eng, int toy, double *nll, double *grad);
+/* gf_set_params and gf_nll (grad null) or gf_nll_grad in one call. */
+int gf_nll_at(gf_engine *eng, int toy, const double *params, int n, double *nll, double *grad);
 /* All toys in one launch sequence: P[n_toys][n_params] -> nll[n_toys], grad[n_toys][n_grad] (grad may be NULL).
  * active[n_toys] (may be NULL) skips toys whose entry is 0. */
 int gf_nll_batch(gf_engine *eng, int n_toys, const double *P, const int32_t *active, double *nll, double *grad);
