@@ -217,7 +217,8 @@ class Engine:
 
     def eval_events(self, metric: int = A.GF_METRIC_PROB, toy: int = 0) -> np.ndarray:
         n = self._n_events.get(toy, 0)
-        out = np.zeros(max(1, n))
+        # not zeroed first: the copy writes all n values, and freshly mapped pages triple its time (8 MB: 188 against 52 us)
+        out = np.empty(max(1, n))
         self._check(self._L.gf_eval_events(self._h, toy, 0, metric, out.ctypes.data_as(A._f64p), n))
         return out[:n]
 
