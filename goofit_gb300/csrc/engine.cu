@@ -1212,6 +1212,7 @@ int updateAmpCaches(gf_engine *e) {
         maxpts = std::max<int64_t>(maxpts, ampPoints(e, k));
     const int64_t bn    = std::min<int64_t>((maxpts + ab - 1) / ab, (int64_t)std::max(1, e->sm_count) * 16);
     const size_t gbytes = sizeof(double) * (size_t)NTILE * e->gram_blocks * PM2;
+    bool chained = anyData; // the stream's last operation is gf_amp
     for(int t = 0; t < NT && r == cudaSuccess; ++t) {
         if(!normDirty[t])
             continue;
@@ -1229,9 +1230,12 @@ int updateAmpCaches(gf_engine *e) {
             // GF_GRAM_TEST_STALL_STAGE (tests of the failure path): the wait for that tile runs out
             const char *stall = std::getenv("GF_GRAM_TEST_STALL_STAGE");
             a.gram_stall      = stall && *stall ? std::atoi(stall) : -1;
-            r = launch(e->mod.ampg, dim3((unsigned)e->gram_ctas, 1, (unsigned)NAN_), dim3(ab), e->plan.gram_smem, e->stream, a);
+            // programmatically chained: gf_amp (when it ran just before) overlaps the integrals, and they the sum's launch
+            r = launch(e->mod.ampg, dim3((unsigned)e->gram_ctas, 1, (unsigned)NAN_), dim3(ab), e->plan.gram_smem, e->stream, a,
+                       e->use_pdl && chained);
+            chained = false;
             if(r == cudaSuccess)
-                r = launch(e->mod.ampg_sum, dim3((unsigned)e->plan.gram_entries), dim3(128), 0, e->stream, a);
+                r = launch(e->mod.ampg_sum, dim3((unsigned)e->plan.gram_entries), dim3(128), 0, e->stream, a, e->use_pdl);
             if(r == cudaSuccess)
                 r = cudaStreamSynchronize(e->stream);
             if(r != cudaSuccess)

@@ -296,6 +296,7 @@ struct GfGram {
 extern "C" __global__ void __launch_bounds__(128) gf_ampng_sum(const GfArgs a) {
     __shared__ double red[4];
     double s = 0.0;
+    gf_pdl_wait();
     for(int b = threadIdx.x; b < a.gram_ctas; b += 128)
         s += a.gpart[(i64)blockIdx.x * a.gram_ctas + b];
 #pragma unroll
