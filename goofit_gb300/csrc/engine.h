@@ -59,7 +59,7 @@ struct GfArgs {
     unsigned long long gram_ns;
     int gram_ctas;
     int gram_stall;       // test of the failure path: the tile whose wait runs out (-1: none)
-    alignas(16) unsigned char rec[1024];
+    alignas(16) unsigned char rec[512];
     const void *p0[192];  // toy 0: observable columns, bin-offset columns, amplitude columns (one toy only)
 };
 

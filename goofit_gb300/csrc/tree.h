@@ -172,14 +172,14 @@ struct NormLayout {
     // no systematic rounding of N
     struct Analytic {
         int node = -1, kind = 0, slotN = -1, slotNL = -1;
-        std::vector<std::pair<int, int>> dN; // (gradient slot, record index of the high part; the low part follows)
+        std::vector<std::pair<int, int>> dN; // (gradient slot, record index)
     };
     int npr = 0; // record length
     std::vector<Analytic> analytic;
     int nq = 0;                                        // numeric slots per toy
     std::vector<int> qN;                               // per numeric node q: slot of N
     std::vector<int> qNL;                              // per numeric node q: slot of the low part of N
-    std::vector<std::vector<std::pair<int, int>>> qdN; // per q: (gradient slot, slot of dN's high part, the low part follows)
+    std::vector<std::vector<std::pair<int, int>>> qdN; // per q: (gradient slot, slot of dN)
 };
 NormLayout norm_layout(const Tree &t);
 
