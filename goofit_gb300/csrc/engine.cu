@@ -484,6 +484,7 @@ int buildLayout(gf_engine *e) {
     chk(dalloc(e, e->d_dgrid, std::max<size_t>(1, ngrid)));
     chk(dalloc(e, e->d_gram, (size_t)NT * std::max(1, NTILE) * e->gram_blocks * std::max(1, 2 * e->plan.gram_pairs_max)));
     chk(dalloc(e, e->d_dirty, NT));
+    e->dirty_set = false;
     if(e->plan.gram_tc) {
         chk(dalloc(e, e->d_gpart, (size_t)e->gram_ctas * e->plan.gram_entries, false));
         if(rc == GF_OK && (cudaHostAlloc((void **)&e->h_gout, sizeof(double) * (e->plan.gram_entries + 1),
@@ -1133,11 +1134,66 @@ int ensureScratch(gf_engine *e) {
     return GF_OK;
 }
 
+// the mark of a word that no launch has written yet: a signalling NaN that no arithmetic result, status or zero equals
+static constexpr uint64_t kRowUnset = 0x7ff40000dead0001ull;
+
+// The integrals of toy e->int_toy from the entries that gf_ampng_sum wrote (the launch has ended, or the words are awaited:
+// every entry is written once over kRowUnset).  An entry still unset after the stream's end was never written.
+int readIntegrals(gf_engine *e) {
+    const gf::Tree &T = e->tree;
+    const int NAN_    = T.n_amp_nodes();
+    GfToy &ty         = e->toys[e->int_toy];
+    e->int_toy        = -1;
+    const uint64_t *w = reinterpret_cast<const uint64_t *>(e->h_gout);
+    for(int q = 0, ended = 0; q < e->plan.gram_entries; ++q)
+        for(unsigned spins = 1; __atomic_load_n(w + q, __ATOMIC_ACQUIRE) == kRowUnset; ++spins) {
+            if(ended)
+                return gf_fail(e, GF_ERR_CUDA, "tensor-core integrals: an entry was not written");
+            if((spins & 127u) == 0) {
+                const cudaError_t r = cudaStreamQuery(e->stream);
+                if(r != cudaSuccess && r != cudaErrorNotReady)
+                    return gf_cuda_check(e, r, "amplitude integrals");
+                ended = r == cudaSuccess;
+            }
+        }
+    if(*reinterpret_cast<volatile int *>(e->h_gout + e->plan.gram_entries))
+        return gf_fail(e, GF_ERR_CUDA, "tensor-core integrals: a bounded wait ran out");
+    for(int k = 0; k < NAN_; ++k) {
+        const int n = T.amp_count(k), nc = ampColumns(T, k), m = 2 * n;
+        const double *G = e->h_gout + e->plan.gram_off[k];
+        // X_u conj(X_v) summed: Re = G(re u, re v) + G(im u, im v), Im = G(im u, re v) - G(re u, im v)
+        auto ent = [&](int u, int v, double &re, double &im) {
+            re = G[(size_t)(2 * u) * m + 2 * v] + G[(size_t)(2 * u + 1) * m + 2 * v + 1];
+            im = G[(size_t)(2 * u + 1) * m + 2 * v] - G[(size_t)(2 * u) * m + 2 * v + 1];
+        };
+        std::vector<double> I(2 * (size_t)n * n, 0.0), H(2 * (size_t)std::max(1, nc - n) * n, 0.0);
+        for(int i = 0; i < n; ++i)
+            for(int j = i; j < n; ++j) {
+                double re, im;
+                ent(i, j, re, im);
+                if(i == j)
+                    im = 0.0;
+                I[2 * (i * n + j)]     = re;
+                I[2 * (i * n + j) + 1] = im;
+                I[2 * (j * n + i)]     = re;
+                I[2 * (j * n + i) + 1] = -im;
+            }
+        for(int d = 0; d < nc - n; ++d)
+            for(int b = 0; b < n; ++b)
+                ent(n + d, b, H[2 * (d * n + b)], H[2 * (d * n + b) + 1]);
+        ty.amp_I[k] = std::move(I);
+        ty.amp_H[k] = std::move(H);
+    }
+    ty.norm_valid = true;
+    return GF_OK;
+}
+
 // Rebuilds the resonance amplitude caches and the normalisation integrals of the active toys whose
 // resonance or efficiency parameters changed since the last build (Amp3Body::normalize's redoIntegral
 // logic, src/PDFs/physics/Amp3Body.cu:263-330).  Runs outside the captured evaluation graph; the
-// evaluations that follow read the caches and the host copies of the integrals.
-int updateAmpCaches(gf_engine *e) {
+// evaluations that follow read the caches and the host copies of the integrals.  defer (one toy): returns once the
+// integrals are enqueued; e->int_toy is then 0 and the caller reads them (readIntegrals) after its own launch.
+int updateAmpCaches(gf_engine *e, bool defer = false) {
     const gf::Tree &T = e->tree;
     const int NAN_    = T.n_amp_nodes();
     if(NAN_ == 0)
@@ -1194,8 +1250,11 @@ int updateAmpCaches(gf_engine *e) {
         return rc;
     GfArgs a      = makeArgs(e);
     cudaError_t r = cudaMemcpyAsync(e->d_P, e->h_P, e->pblock_bytes, cudaMemcpyHostToDevice, e->stream);
-    if(r == cudaSuccess)
-        r = cudaMemcpyAsync(e->d_dirty, e->h_dirty, sizeof(int) * NT, cudaMemcpyHostToDevice, e->stream);
+    // one toy: its flag on the device stays set (the kernels that read it run only when it is)
+    if(r == cudaSuccess && (NT > 1 || (anyData && !e->dirty_set))) {
+        r            = cudaMemcpyAsync(e->d_dirty, e->h_dirty, sizeof(int) * NT, cudaMemcpyHostToDevice, e->stream);
+        e->dirty_set = NT == 1;
+    }
     if(r == cudaSuccess && anyData && nk > 0)
         r = launch(e->mod.ampc, dim3((unsigned)e->plan.amp_terms, NT), dim3(32), 0, e->stream, a);
     if(r == cudaSuccess && anyData) {
@@ -1230,6 +1289,8 @@ int updateAmpCaches(gf_engine *e) {
         if(tc) {
             int *err = reinterpret_cast<int *>(e->h_gout + e->plan.gram_entries);
             *err     = 0;
+            for(int q = 0; q < e->plan.gram_entries; ++q)
+                reinterpret_cast<uint64_t *>(e->h_gout)[q] = kRowUnset;
             // GF_GRAM_TEST_STALL_STAGE (tests of the failure path): the wait for that tile runs out
             const char *stall = std::getenv("GF_GRAM_TEST_STALL_STAGE");
             a.gram_stall      = stall && *stall ? std::atoi(stall) : -1;
@@ -1239,40 +1300,16 @@ int updateAmpCaches(gf_engine *e) {
             chained = false;
             if(r == cudaSuccess)
                 r = launch(e->mod.ampg_sum, dim3((unsigned)e->plan.gram_entries), dim3(128), 0, e->stream, a, e->use_pdl);
+            ty.amp_params = snap[t];
+            e->int_toy    = t;
+            if(defer && r == cudaSuccess)
+                return GF_OK;
             if(r == cudaSuccess)
                 r = cudaStreamSynchronize(e->stream);
             if(r != cudaSuccess)
                 break;
-            if(*reinterpret_cast<volatile int *>(err))
-                return gf_fail(e, GF_ERR_CUDA, "tensor-core integrals: a bounded wait ran out");
-            for(int k = 0; k < NAN_; ++k) {
-                const int n = T.amp_count(k), nc = ampColumns(T, k), m = 2 * n;
-                const double *G = e->h_gout + e->plan.gram_off[k];
-                // X_u conj(X_v) summed: Re = G(re u, re v) + G(im u, im v), Im = G(im u, re v) - G(re u, im v)
-                auto ent = [&](int u, int v, double &re, double &im) {
-                    re = G[(size_t)(2 * u) * m + 2 * v] + G[(size_t)(2 * u + 1) * m + 2 * v + 1];
-                    im = G[(size_t)(2 * u + 1) * m + 2 * v] - G[(size_t)(2 * u) * m + 2 * v + 1];
-                };
-                std::vector<double> I(2 * (size_t)n * n, 0.0), H(2 * (size_t)std::max(1, nc - n) * n, 0.0);
-                for(int i = 0; i < n; ++i)
-                    for(int j = i; j < n; ++j) {
-                        double re, im;
-                        ent(i, j, re, im);
-                        if(i == j)
-                            im = 0.0;
-                        I[2 * (i * n + j)]     = re;
-                        I[2 * (i * n + j) + 1] = im;
-                        I[2 * (j * n + i)]     = re;
-                        I[2 * (j * n + i) + 1] = -im;
-                    }
-                for(int d = 0; d < nc - n; ++d)
-                    for(int b = 0; b < n; ++b)
-                        ent(n + d, b, H[2 * (d * n + b)], H[2 * (d * n + b) + 1]);
-                ty.amp_I[k] = std::move(I);
-                ty.amp_H[k] = std::move(H);
-            }
-            ty.amp_params = snap[t];
-            ty.norm_valid = true;
+            if((rc = readIntegrals(e)))
+                return rc;
             continue;
         }
         if(r == cudaSuccess)
@@ -1480,7 +1517,6 @@ struct NvtxScope {
 
 // The host's mark of a one-launch row word not yet written: a signalling-NaN bit pattern, which no arithmetic
 // result (quiet NaNs only) and no status or zero the kernel stores can equal.
-static constexpr uint64_t kRowUnset = 0x7ff40000dead0001ull;
 
 // A row word written by the device into mapped host memory (one aligned 8-byte store), read as a double.
 static inline double wordValue(const uint64_t *p) {
@@ -1510,7 +1546,12 @@ int gf_run(gf_engine *e, bool grad, int, int) {
         return rc;
     {
         NvtxScope s("gf_amplitude_caches");
-        if((rc = updateAmpCaches(e)))
+        // one launch whose only amplitude PDF is the root: its normalisation is applied on the host, so the launch does
+        // not wait for the integrals, and the host reads them after the rows (no synchronisation in between: 12 us of a
+        // call that rebuilds them)
+        e->int_toy = -1;
+        if((rc = updateAmpCaches(e, fusedPath(e) && !e->tune_pending && e->plan.factor_root && e->tree.n_amp_nodes() == 1 &&
+                                        e->tree.amp_node(0) == 0)))
             return rc;
     }
     fillRecords(e);
@@ -1660,6 +1701,11 @@ int gf_run(gf_engine *e, bool grad, int, int) {
             ++c;
         }
         e->timing_pending = true;
+        if(e->int_toy >= 0) {
+            if((rc = readIntegrals(e)))
+                return rc;
+            fillRecords(e); // the root's normalisation
+        }
         double *o = e->h_out;
         o[0]      = sum[0];
         for(int k = 1; k < NGp; ++k)

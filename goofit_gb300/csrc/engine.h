@@ -156,6 +156,8 @@ struct gf_engine {
     double *d_gram = nullptr;    // integral partials [toy][tile][CTA][2 * pairs]
     double *h_gram = nullptr;
     int *d_dirty = nullptr, *h_dirty = nullptr;
+    bool dirty_set = false; // one toy: d_dirty holds its flag, set
+    int int_toy    = -1;    // the toy whose integrals are enqueued and not yet read
     // parameter-only constants of the Amp3Body resonances, 8 bytes each; kept with the amplitude caches they were
     // built with, across layout rebuilds (freed with the tree or the toys)
     unsigned long long *d_ampc = nullptr;
