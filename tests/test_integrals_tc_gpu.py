@@ -1,5 +1,5 @@
 """gf_ampng (amplitudes and tensor-core contraction in one pass) against the CUDA-core integrals of the same engine, over
-its layouts: slices of 32 and 64 real columns, weighted (Amp3Body) and unweighted (Amp4Body), 1 to 8 amplitudes, with
+its layouts: slices of 32 and 64 real columns, weighted (Amp3Body) and unweighted (Amp4Body), 1 to 31 amplitudes, with
 and without derivative columns, and point counts around one tile of 128."""
 import numpy as np
 import pytest
@@ -24,6 +24,23 @@ def _three(n_res, floated, bins):
     return pdf, np.vstack([x, np.arange(x.shape[1])]), None
 
 
+def _many(n_res, floated, bins):
+    """n_res resonances: value columns up to the widest that one slice holds."""
+    m12, m13 = G.Observable("m12", 0.0, 3.0), G.Observable("m13", 0.0, 3.0)
+    m12.setNumBins(bins)
+    m13.setNumBins(bins)
+    d = G.DecayInfo3()
+    d.motherMass, d.daug1Mass, d.daug2Mass, d.daug3Mass = W.C3_M, W.C3_MK, W.C3_MPI, W.C3_MPI0
+    d.meson_radius, d.mother_meson_radius = 1.5, 5.0
+    for k in range(n_res):
+        m, w = G.Variable(f"m{k}", 0.7 + 0.03 * k), G.Variable(f"w{k}", 0.1)
+        m.setFixed(k >= floated)
+        d.add_resonance(G.RBW(f"r{k}", G.Variable(f"re{k}", 1.0, 0.01, 0, 0), G.Variable(f"im{k}", 0.1 * (k % 5), 0.01, 0, 0), m, w,
+                              k % 2, int((G.PAIR_12, G.PAIR_13, G.PAIR_23)[k % 3])))
+    pdf = G.Amp3Body("p", m12, m13, G.EventNumber("eventNumber"), d)
+    return pdf, _three(2, 0, 40)[1], None
+
+
 def _four(floated, points):
     pdf = W.c5_model(1000, float_lineshapes=floated)[0]
     ev = phasespace.norm_events(W.C5_M, W.C5_MASSES, 1500 + points, 11)
@@ -42,7 +59,7 @@ def _evaluate(make, args):
     eng.upload(events)
     p = np.array([v.value for v in params]) * (1 + 0.01 * np.cos(np.arange(len(params))) * np.array(mask))
     nll, grad = eng.nll_grad(p)
-    n = args[0] if make is _three else 6
+    n = 6 if make is _four else args[0]
     out = nll, grad, eng.amp3_integrals(0, n), n
     eng.close()
     return out
@@ -51,7 +68,7 @@ def _evaluate(make, args):
 @pytest.mark.parametrize("make,args", [
     (_three, (8, 0, 61)), (_three, (8, 4, 61)), (_three, (8, 8, 40)), (_three, (1, 1, 40)), (_three, (3, 2, 19)),
     (_four, (False, 1000)), (_four, (True, 1)), (_four, (True, 127)), (_four, (True, 128)), (_four, (True, 129)),
-    (_four, (True, 60001)),
+    (_four, (True, 60001)), (_many, (9, 0, 40)), (_many, (16, 0, 40)), (_many, (17, 2, 40)), (_many, (31, 1, 40)),
 ])
 def test_one_pass_integrals_match_the_cuda_core_integrals(make, args, monkeypatch):
     monkeypatch.delenv("GF_GRAM", raising=False)
