@@ -2095,7 +2095,7 @@ int gf_upload_events(gf_engine *e, int toy, const double *soa, int64_t n) {
             direct = true;
         }
         cudaGetLastError();
-        if(!direct && !(st && st[0] == '1') && readsInPlace(e, soa, n * NO)) {
+        if(!direct && n > 0 && !(st && st[0] == '1') && pa.type == cudaMemoryTypeUnregistered && readsInPlace(e, soa, n * NO)) {
             src    = soa;
             direct = true;
         }
