@@ -8,6 +8,7 @@
 // evaluation kind that runs   H2D(params) -> conv tables -> grid sums ->
 // event pass -> D2H(result)   in a single graph launch.
 #include "engine.h"
+#include "gram_tc.h"
 #include "rtc.h"
 
 #include <nvtx3/nvToolsExt.h>
@@ -488,8 +489,7 @@ int buildLayout(gf_engine *e) {
     e->dirty_set = false;
     if(e->plan.gram_tc) {
         chk(dalloc(e, e->d_gpart, (size_t)e->gram_ctas * e->plan.gram_entries, false));
-        if(rc == GF_OK && (cudaHostAlloc((void **)&e->h_gout, sizeof(double) * (e->plan.gram_entries + 1),
-                                         cudaHostAllocMapped) != cudaSuccess ||
+        if(rc == GF_OK && (cudaHostAlloc((void **)&e->h_gout, sizeof(double) * e->plan.gram_entries, cudaHostAllocMapped) != cudaSuccess ||
                            cudaHostGetDevicePointer((void **)&e->d_gout, e->h_gout, 0) != cudaSuccess))
             rc = gf_fail(e, GF_ERR_OOM, "cudaHostAlloc");
     }
@@ -591,7 +591,6 @@ GfArgs makeArgs(gf_engine *e) {
     a.gram_ns     = e->gram_ns ? e->gram_ns : 2000000000ull;
     a.gram_stall  = -1;
     a.gout        = e->d_gout;
-    a.gerr        = e->d_gout ? reinterpret_cast<int *>(e->d_gout + e->plan.gram_entries) : nullptr;
     a.gtoy        = 0;
     a.chunk       = e->chunk;
     a.nevt0       = e->toys.empty() ? 0 : e->toys[0].n;
@@ -1139,7 +1138,8 @@ int ensureScratch(gf_engine *e) {
 static constexpr uint64_t kRowUnset = 0x7ff40000dead0001ull;
 
 // The integrals of toy e->int_toy from the entries that gf_ampng_sum wrote (the launch has ended, or the words are awaited:
-// every entry is written once over kRowUnset).  An entry still unset after the stream's end was never written.
+// every entry is written once over kRowUnset).  An entry still unset after the stream's end was never written; one that
+// holds kGramStopped stands for a CTA whose bounded wait ran out.
 int readIntegrals(gf_engine *e) {
     const gf::Tree &T = e->tree;
     const int NAN_    = T.n_amp_nodes();
@@ -1157,8 +1157,9 @@ int readIntegrals(gf_engine *e) {
                 ended = r == cudaSuccess;
             }
         }
-    if(*reinterpret_cast<volatile int *>(e->h_gout + e->plan.gram_entries))
-        return gf_fail(e, GF_ERR_CUDA, "tensor-core integrals: a bounded wait ran out");
+    for(int q = 0; q < e->plan.gram_entries; ++q)
+        if(w[q] == gf::kGramStopped)
+            return gf_fail(e, GF_ERR_CUDA, "tensor-core integrals: a bounded wait ran out");
     for(int k = 0; k < NAN_; ++k) {
         const int n = T.amp_count(k), nc = ampColumns(T, k), m = 2 * n;
         const double *G = e->h_gout + e->plan.gram_off[k];
@@ -1288,8 +1289,6 @@ int updateAmpCaches(gf_engine *e, bool defer = false) {
         ty.amp_I.assign(NAN_, {});
         ty.amp_H.assign(NAN_, {});
         if(tc) {
-            int *err = reinterpret_cast<int *>(e->h_gout + e->plan.gram_entries);
-            *err     = 0;
             for(int q = 0; q < e->plan.gram_entries; ++q)
                 reinterpret_cast<uint64_t *>(e->h_gout)[q] = kRowUnset;
             // GF_GRAM_TEST_STALL_STAGE (tests of the failure path): the wait for that tile runs out
@@ -1703,9 +1702,9 @@ int gf_run(gf_engine *e, bool grad, int, int) {
         }
         e->timing_pending = true;
         if(e->int_toy >= 0) {
-            if((rc = readIntegrals(e)))
-                return rc;
-            fillRecords(e); // the root's normalisation
+            rc = readIntegrals(e); // a failure is returned below, once a stopped launch has been cleaned up
+            if(rc == GF_OK)
+                fillRecords(e); // the root's normalisation
         }
         double *o = e->h_out;
         o[0]      = sum[0];
@@ -1744,7 +1743,7 @@ int gf_run(gf_engine *e, bool grad, int, int) {
         e->h_out[1] = 8.0;
         return gf_fail(e, GF_ERR_TIMEOUT, "a grid barrier wait of the one-launch evaluation ran out");
     }
-    return GF_OK;
+    return rc;
 }
 
 extern "C" {

@@ -54,8 +54,7 @@ struct GfArgs {
     const int *ksort;     // one-launch tabulated path: toy 0's bin offsets sorted by bin (null: read kcol)
     const void *ampc;     // [toy][term][k] parameter-only constants of the Amp3Body resonances (gf_ampc)
     double *gpart;        // tensor-core integrals: [entry][CTA] partials of gram_ctas CTAs, their sums in page-locked
-    double *gout;         // memory, the error word and the longest wait for a tile's MMAs
-    int *gerr;
+    double *gout;         // memory, and the longest wait for a tile's MMAs
     unsigned long long gram_ns;
     int gram_ctas;
     int gram_stall;       // test of the failure path: the tile whose wait runs out (-1: none)
@@ -167,8 +166,8 @@ struct gf_engine {
     std::vector<int64_t> norm_n;
     double **d_nevt = nullptr;
     long long *d_nnorm = nullptr;
-    // tensor-core integrals (mixed precision, gf_ampng): CTAs, their FP64 partials, and in one mapped page-locked block
-    // the summed entries followed by the error word
+    // tensor-core integrals (mixed precision, gf_ampng): CTAs, their FP64 partials, and the summed entries in mapped
+    // page-locked memory
     int gram_ctas      = 0;
     double *d_gpart    = nullptr;
     double *h_gout = nullptr, *d_gout = nullptr;

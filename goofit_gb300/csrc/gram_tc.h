@@ -28,8 +28,10 @@
 // tensor memory beside it (registers would cost the amplitudes their occupancy).  The MMAs of one tile run while the
 // threads evaluate the amplitudes of the next, so one operand buffer is enough.
 //
-// Every wait is bounded: a wait that runs out sets *gerr; the CTA stops issuing work, waits (bounded) for what it
-// issued, frees its tensor memory and returns.
+// Every wait is bounded: after a wait that runs out the CTA stops issuing work, waits (bounded) for what it issued, frees
+// its tensor memory and writes kGramStopped in the place of its partials, and the sums hand it on.  The host may read the
+// sums while the launch ends, so the failure has to stand in the words that it waits for: a flag beside them, written by
+// another kernel, need not be visible when they are.
 #pragma once
 
 #include <cstddef>
@@ -37,6 +39,8 @@
 namespace gf {
 
 constexpr int kGramThreads = 128;
+// the partials of a CTA whose wait ran out, and the sums over them: a signalling NaN, which no arithmetic gives
+constexpr unsigned long long kGramStopped = 0x7ff40000dead0002ull;
 
 // real columns per slice for a node of nc complex columns (0: more than 64 real columns, no tensor-core kernel) and
 // value columns per slice for n amplitudes
@@ -59,6 +63,7 @@ inline size_t gram_smem(int w, int wn, bool weighted) {
 }
 
 const char *const kGramSource = R"CUDA(
+#define GF_GRAM_STOPPED 0x7ff40000dead0002ull /* kGramStopped */
 __device__ __forceinline__ unsigned gf_s32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void gf_tc_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void gf_tc_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -246,16 +251,14 @@ struct GfGram {
         return true;
     }
     // Ends the CTA's pass: its sums over the slices, in FP64, to out[entry * gridDim.x + blockIdx.x]; frees the tensor
-    // memory.  A wait that ran out (here or in tile) is reported in *err.
-    __device__ __forceinline__ void end(bool ok, double *out, int *err) {
+    // memory.  After a wait that ran out (here or in tile) GF_GRAM_STOPPED in their place.
+    __device__ __forceinline__ void end(bool ok, double *out) {
         if(ok && last >= 0) {
             ok = wait(last);
             if(ok)
                 drain();
         }
         if(__syncthreads_or(!ok)) {
-            if(threadIdx.x == 0)
-                *reinterpret_cast<volatile int *>(err) = 1;
             // the last committed MMAs must have ended before the tensor memory goes away (2 s, whatever the limit)
             if(last >= 0)
                 gf_mbar_wait(&sh->mbar, (unsigned)(last & 1), 2000000000ull);
@@ -280,8 +283,11 @@ struct GfGram {
         gf_tc_after();
         if(threadIdx.x < 32)
             asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS) : "memory");
-        if(!ok)
+        if(!ok) {
+            for(int q = threadIdx.x; q < 4 * NC * NA; q += 128)
+                reinterpret_cast<unsigned long long *>(out)[(i64)q * gridDim.x + blockIdx.x] = GF_GRAM_STOPPED;
             return;
+        }
         for(int q = threadIdx.x; q < 4 * NC * NA; q += 128) {
             const int i = q / (2 * NA), j = q % (2 * NA);
             double t = 0.0;
@@ -292,21 +298,29 @@ struct GfGram {
     }
 };
 
-// entry blockIdx.x of every node's G: the sum over the CTAs' partials, FP64
+// entry blockIdx.x of every node's G: the sum over the CTAs' partials, FP64; GF_GRAM_STOPPED when a CTA stopped
 extern "C" __global__ void __launch_bounds__(128) gf_ampng_sum(const GfArgs a) {
     __shared__ double red[4];
     double s = 0.0;
+    bool stopped = false;
     gf_pdl_wait();
-    for(int b = threadIdx.x; b < a.gram_ctas; b += 128)
-        s += a.gpart[(i64)blockIdx.x * a.gram_ctas + b];
+    for(int b = threadIdx.x; b < a.gram_ctas; b += 128) {
+        const double v = a.gpart[(i64)blockIdx.x * a.gram_ctas + b];
+        stopped |= (unsigned long long)__double_as_longlong(v) == GF_GRAM_STOPPED;
+        s += v;
+    }
 #pragma unroll
     for(int o = 16; o > 0; o >>= 1)
         s += __shfl_xor_sync(0xffffffffu, s, o);
     if((threadIdx.x & 31) == 0)
         red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if(threadIdx.x == 0)
-        a.gout[blockIdx.x] = (red[0] + red[1]) + (red[2] + red[3]);
+    stopped = __syncthreads_or(stopped);
+    if(threadIdx.x == 0) {
+        if(stopped)
+            reinterpret_cast<unsigned long long *>(a.gout)[blockIdx.x] = GF_GRAM_STOPPED;
+        else
+            a.gout[blockIdx.x] = (red[0] + red[1]) + (red[2] + red[3]);
+    }
 }
 )CUDA";
 
