@@ -1554,7 +1554,10 @@ int gf_run(gf_engine *e, bool grad, int, int) {
                                         e->tree.amp_node(0) == 0)))
             return rc;
     }
-    fillRecords(e);
+    // with integrals in flight the records stand as the rebuild filled them, from the same parameters: the copy of their
+    // page-locked block to the device may still be reading it
+    if(e->int_toy < 0)
+        fillRecords(e);
     if(e->tune_pending) {
         NvtxScope s("gf_autotune");
         e->tune_pending = false;
