@@ -1052,8 +1052,10 @@ int64_t ampPoints(const gf_engine *e, int k) {
 int64_t ampStride(const gf_engine *e, int k) { return (std::max<int64_t>(1, ampPoints(e, k)) + 3) / 4 * 4; }
 
 // Bytes the store mode keeps for amplitude derivatives and normalisation points: the derivative columns of every
-// toy's events (npad events each) and the normalisation scratch columns.
-size_t ampStoreBytes(const gf_engine *e, int64_t npad) {
+// toy's events (npad events each), and the normalisation scratch columns where gf_ampn writes them (gf_ampng sums the
+// points as it evaluates them and keeps none).  asColumns: with scratch columns in any case, which is what the automatic
+// mode's budget is measured against (so that a budget chooses the same mode whichever kernel forms the integrals).
+size_t ampStoreBytes(const gf_engine *e, int64_t npad, bool asColumns = false) {
     const gf::Tree &T = e->tree;
     const size_t rs   = rsize(e);
     size_t nd = 0, scr = 0;
@@ -1062,7 +1064,8 @@ size_t ampStoreBytes(const gf_engine *e, int64_t npad) {
         for(auto &th : T.amp_theta(k))
             ndk += (int)th.amps.size();
         nd += (size_t)ndk;
-        scr += (size_t)ampStride(e, k) * ((T.amp_count(k) + ndk) * 2 * rs + rs);
+        if(asColumns || !e->plan.gram_tc)
+            scr += (size_t)ampStride(e, k) * ((T.amp_count(k) + ndk) * 2 * rs + rs);
     }
     return (size_t)e->n_toys * (size_t)npad * nd * 2 * rs + scr;
 }
@@ -1085,7 +1088,7 @@ void decideAmpMode(gf_engine *e, int64_t npad) {
                 }
                 budget = fr / 4;
             }
-            rc = ampStoreBytes(e, npad) > budget;
+            rc = ampStoreBytes(e, npad, true) > budget;
         }
     }
     e->amp_recompute = rc;

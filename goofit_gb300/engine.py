@@ -264,7 +264,7 @@ class Engine:
 
     def set_amp_mode(self, mode: str, budget_bytes: int = 0) -> None:
         """Amplitude derivatives 'store'd per event and normalisation point, 'recompute'd where they are used,
-        or 'auto' (recompute when storing would take more than budget_bytes; 0: a quarter of the free device
+        or 'auto' (recompute when columns of both would take more than budget_bytes; 0: a quarter of the free device
         memory).  Before the first upload."""
         m = {"auto": A.GF_AMP_AUTO, "store": A.GF_AMP_STORE, "recompute": A.GF_AMP_RECOMPUTE}[mode]
         self._check(self._L.gf_set_amp_mode(self._h, m, int(budget_bytes)))

@@ -219,11 +219,13 @@ int gf_set_wait_limit(gf_engine *eng, uint64_t ns);
 int gf_set_gram_wait_limit(gf_engine *eng, uint64_t ns);
 
 /* Where the derivatives of the amplitudes by floated resonance / line-shape parameters live (Amp3Body, Amp4Body).
-   GF_AMP_STORE: per-event columns and per-normalisation-point scratch columns, as the reference caches its
-   line shapes, spin factors and amplitudes (src/PDFs/physics/Amp4Body.cu:348-395).  GF_AMP_RECOMPUTE: only the
+   GF_AMP_STORE: per-event columns, as the reference caches its line shapes, spin factors and amplitudes
+   (src/PDFs/physics/Amp4Body.cu:348-395), and per-normalisation-point scratch columns (FP64, or more than 32 columns:
+   the mixed engine's integrals are otherwise summed as the points are evaluated).  GF_AMP_RECOMPUTE: only the
    amplitude values are cached per event; the gradient pass recomputes dA/dt per event, and the integrals are
    reduced from amplitudes recomputed at every normalisation point (no per-point storage).  GF_AMP_AUTO (the
-   default) recomputes when storing would take more than budget_bytes (0: a quarter of the free device memory).
+   default) recomputes when per-event and scratch columns would take more than budget_bytes (0: a quarter of the free
+   device memory), scratch columns counted whether or not the integrals take them.
    Takes effect at the next gf_set_tree, or at the first gf_upload_events after it; GF_ERR_STATE once events
    are uploaded. */
 enum gf_amp_mode { GF_AMP_AUTO = 0, GF_AMP_STORE = 1, GF_AMP_RECOMPUTE = 2 };
@@ -231,8 +233,8 @@ int gf_set_amp_mode(gf_engine *eng, int mode, int64_t budget_bytes);
 /* 1: the engine recomputes amplitude derivatives, 0: it stores them (or the tree has none), -1: not decided yet
    (no events uploaded since gf_set_tree). */
 int gf_amp_recomputing(const gf_engine *eng);
-/* Device bytes the store mode keeps for the derivative columns of the uploaded events and the normalisation
-   scratch columns (what the recompute mode does without); 0 without amplitude nodes or events. */
+/* Device bytes the store mode keeps for the derivative columns of the uploaded events and, where the integrals take
+   them, the normalisation scratch columns (what the recompute mode does without); 0 without amplitude nodes or events. */
 int64_t gf_amp_store_bytes(const gf_engine *eng);
 
 /* Launch-shape autotuner (the counterpart of the reference's grain-size sweep, scripts/find_optimal.py): times
