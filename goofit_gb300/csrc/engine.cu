@@ -1887,8 +1887,10 @@ int gf_set_tree(gf_engine *e, const gf_node *nodes, int n_nodes, const gf_observ
 // sizes the event chunks from the gradient event kernel's occupancy.
 static int compileTree(gf_engine *e) {
     e->batch_kernels = e->n_toys > 1;
+    gf::Shapes sh    = e->shapes;
+    sh.sms           = std::max(1, e->sm_count);
     try {
-        e->plan = gf::generate_kernels(e->tree, e->precision == GF_MIXED, e->block, e->batch_kernels, e->shapes);
+        e->plan = gf::generate_kernels(e->tree, e->precision == GF_MIXED, e->block, e->batch_kernels, sh);
     } catch(std::exception &ex) {
         return gf_fail(e, GF_ERR_BAD_TREE, ex.what());
     }

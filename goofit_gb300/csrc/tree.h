@@ -241,10 +241,11 @@ struct KernelPlan {
 
 // batch: kernels shaped for many toys per launch (fewer, larger table and grid CTAs)
 // Launch shapes the autotuner varies (0: the generator's default): table k-tiles per staged model and resolution
-// (batches of toys), numeric-grid bins per CTA.
+// (batches of toys), numeric-grid bins per CTA.  sms: the device's SMs (a GB300's where no device is asked).
 struct Shapes {
     int conv_kp  = 0;
     int grid_bpb = 0;
+    int sms      = 152;
 };
 KernelPlan generate_kernels(const Tree &t, bool mixed, int evt_block, bool batch, const Shapes &shapes = Shapes());
 
