@@ -1,5 +1,5 @@
-"""Floated four-body line shapes of the mixed engine (gf_lineshape_k, and the dual numbers of shapes whose thresholds move
-with the event) against the FP64 engine: at and just above the thresholds of the pairs (1,2) and (3,4), and over orbital
+"""Four-body line shapes of the mixed engine (floated ones: gf_lineshape_k, and the dual numbers of shapes whose thresholds
+move with the event) against the FP64 engine: at and just above the thresholds, and over orbital
 angular momenta, form factors, constant widths, poles below threshold and daughter combinations.  Amplitudes of one line
 shape and no spin factor, so that the cached wave is the line shape itself."""
 import numpy as np
@@ -90,6 +90,49 @@ def test_at_and_just_above_the_threshold():
     want = -np.log(probs).sum() + 20 * (np.log(r64.normalize()[1][0]) - np.log(eng.normalize()[1][0]))
     # per event: FP32 log of a density of relative error 1e-6
     assert abs((nll - some.nll(p)) - want) <= 20 * 1e-5
+
+
+def test_fixed_shapes_at_and_just_above_the_threshold():
+    shapes = [(RBW, 0.775, 0.149, 0, P.M_12, FF.BL_Prime), (RBW, 0.892, 0.1, 1, P.M_34, FF.BL_Prime),
+              (RBW, 0.6, 0.3, 1, P.M_12, FF.BL2), (RBW, 0.8, 0.3, 2, P.M_34, FF.BL2)]
+    x = _threshold_events()
+    ref, p, _ = _engine("fp64", _model(shapes, floated=False), x, x[:, 20:])
+    eng, _, _ = _engine("mixed", _model(shapes, floated=False), x, x)
+    for a in range(len(shapes)):
+        want, got = ref.amp3_cached_wave(0, a), eng.amp3_cached_wave(0, a)
+        # these shapes subtract in FP32: q^2 is off by 2^-23 s at most, 1e-4 GeV of q at the threshold, against a pole term
+        # of 0.5 GeV^2 and a width term of m Gamma q / q0 < 0.4 GeV q
+        assert np.all(np.abs(got - want) <= 5e-4 * np.abs(want).max()), a
+    nll, grad = eng.nll_grad(p)
+    assert np.isfinite(nll) and np.all(np.isfinite(grad))
+
+
+def _triple_events(cos34):
+    """Events in which daughter 3 moves with the pair (1,2), so that m123 = m12 + m3; where it moves against it, for the
+    other sign of cos34."""
+    m12 = np.linspace(M[0] + M[1] + 0.01, W.C5_M - M[2] - M[3] - 0.2, 200)
+    cl = m12 + M[2]
+    p = np.sqrt((W.C5_M ** 2 - (cl + M[3]) ** 2) * (W.C5_M ** 2 - (cl - M[3]) ** 2)) / (2 * W.C5_M)
+    e3, e4 = M[2] * np.sqrt(1 + (p / cl) ** 2), np.sqrt(M[3] ** 2 + p ** 2)
+    m34 = np.sqrt((e3 + e4) ** 2 - (p * m12 / cl) ** 2)
+    return np.vstack([m12, m34, np.full(200, 0.3), np.full(200, cos34), np.linspace(-3, 3, 200)])
+
+
+@pytest.mark.parametrize("floated", [True, False])
+def test_triples_at_their_threshold(floated):
+    # poles above every event's mass (1.53 GeV): the width vanishes at the threshold, and a pole there would diverge
+    shapes = [(RBW, 1.8, 0.3, 0, P.M_12_3, FF.BL_Prime), (RBW, 1.75, 0.3, 1, P.M_12_3, FF.BL2), (SBW, 1.8, 0.3, 1, P.M_12_3, FF.BL)]
+    x = np.hstack([_triple_events(c) for c in (1.0, -1.0)])
+    near = np.hstack([_triple_events(c) for c in (1 - 1e-9, -1 + 1e-9)])
+    ref, p, _ = _engine("fp64", _model(shapes, floated=False), near, _events(400, 3))
+    eng, _, _ = _engine("mixed", _model(shapes, floated), x, np.hstack([x, _events(400, 3)]))
+    for a in range(len(shapes)):
+        want, got = ref.amp3_cached_wave(0, a), eng.amp3_cached_wave(0, a)
+        # the squared mass from FP32 four-vectors: a few units of 2^-24 M^2, 1e-6 GeV^2, so q is off by up to 1e-3 GeV
+        # there, and the wave by m Gamma q / q0 (the last shape's form factor: q r) over a pole term of 0.7 GeV^2
+        assert np.all(np.isfinite(got)) and np.all(np.abs(got - want) <= 5e-3 * np.abs(want).max()), a
+    nll, grad = eng.nll_grad(p)
+    assert np.isfinite(nll) and np.all(np.isfinite(grad))
 
 
 FORMS = [
