@@ -22,9 +22,10 @@
 // by (group of 8 columns, slice), which makes them A's first N rows, and 64 KB hold a CTA's operands, so that three
 // CTAs stay resident.  Weighted (Amp3Body), B = e x has its own 1024 Wn bytes.
 //
-// Each product takes three MMAs (lo hi + hi lo + hi hi), about 22 significant bits.  The tensor core's FP32
+// Each product takes four MMAs (lo lo + hi lo + lo hi + hi hi).  The tensor core's FP32
 // accumulation rounds towards zero, so an accumulator sums one tile's 32 points per slice only: the small terms first,
-// then four MMAs of large ones.  The tile's accumulator is added to a compensated FP32 pair per entry, which lives in
+// then four MMAs of large ones.  That leaves sums of squares 8 to 9e-8 short; without lo lo, which is positive in each of
+// them, it was 12 to 13e-8 (8 resonances, 794,107 points, the error of a fit's NLL against 64 bits 4.1e-7 -> 3.1e-7).  The tile's accumulator is added to a compensated FP32 pair per entry, which lives in
 // tensor memory beside it (registers would cost the amplitudes their occupancy).  The MMAs of one tile run while the
 // threads evaluate the amplitudes of the next, so one operand buffer is enough.
 //
@@ -88,6 +89,14 @@ __device__ __forceinline__ void gf_tmem_st8(unsigned addr, const float *v) {
                  "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])) : "memory");
 }
 __device__ __forceinline__ void gf_tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// One lane of a converged warp.  Issuing a tile's 16 or 32 MMAs is on the path of all its threads, which meet before and
+// after it; from an elected lane it is shorter than from threadIdx.x == 0 (rebuild of 8 resonances 395 -> 379 us, of the
+// four-body model 928 -> 892 us).
+__device__ __forceinline__ bool gf_elect() {
+    unsigned p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
 struct GfGramShared {
     unsigned long long mbar, never; /* MMAs of a tile; a barrier that nothing arrives on (test of the failure path) */
     unsigned tmem;
@@ -201,14 +210,13 @@ struct GfGram {
             put((storeB ^ sw) + (unsigned)i * 128u, x * e, BBYTES);
     }
     // Shared-memory matrix descriptor: start >> 4 (bits 0-13), leading offset (unused in this layout: 1), stride
-    // between 8-row groups 1024 >> 4 (bits 32-45), version 1 (bits 46-47), 128-byte swizzle (2 in bits 61-63)
-    static __device__ __forceinline__ unsigned long long desc(unsigned at) {
-        return (unsigned long long)((at >> 4) & 0x3FFFu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-    }
-    static __device__ __forceinline__ void mma(unsigned d, unsigned at, unsigned bt, unsigned accumulate) {
-        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                     "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d), "l"(desc(at)), "l"(desc(bt)),
-                     "r"(IDESC), "r"(accumulate) : "memory");
+    // between 8-row groups 1024 >> 4 (bits 32-45), version 1 (bits 46-47), 128-byte swizzle (2 in bits 61-63).  The low word
+    // of base; an operand at an offset adds the offset >> 4 to it.
+    __device__ __forceinline__ unsigned desc() const { return ((base >> 4) & 0x3FFFu) | (1u << 16); }
+    static __device__ __forceinline__ void mma(unsigned d, unsigned a, unsigned b, unsigned accumulate) {
+        asm volatile("{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %4, 0;\n\tmov.b64 da, {%1, %5};\n\tmov.b64 db, {%2, %5};\n\t"
+                     "tcgen05.mma.cta_group::1.kind::tf32 [%0], da, db, %3, p;\n\t}\n" ::"r"(d), "r"(a), "r"(b),
+                     "r"(IDESC), "r"(accumulate), "r"(64u | (1u << 14) | (2u << 29)) : "memory");
     }
     // Tile u: this thread's point (values A, derivatives dA, efficiency e; zeros outside the set).  False on every
     // thread when the wait for the previous tile's MMAs ran out in any.
@@ -230,20 +238,22 @@ struct GfGram {
         gf_tc_before();
         if(__syncthreads_or(!ok))
             return false;
-        if(threadIdx.x == 0) {
+        if(threadIdx.x < 32 && gf_elect()) {
             gf_tc_after();
-            const unsigned bh = WT ? base + 2 * ABYTES : base, bl = WT ? bh + BBYTES : base + ABYTES;
+            const unsigned D = desc();
+            constexpr unsigned AL = ABYTES >> 4, BH = WT ? 2 * AL : 0u, BL = WT ? BH + (BBYTES >> 4) : AL;
 #pragma unroll
             for(int b = 0; b < KB; ++b) {
-                const unsigned oa = b * 16384u, ob = WT ? b * N * 128u : oa, d = tmem + (unsigned)(b * N);
+                const unsigned oa = b * 1024u, ob = WT ? b * N * 8u : oa, d = tmem + (unsigned)(b * N);
 #pragma unroll
                 for(int k = 0; k < 4; ++k) { // 8 points: 32 bytes of every 128-byte row
-                    mma(d, base + oa + 32 * k, bl + ob + 32 * k, k > 0);
-                    mma(d, base + ABYTES + oa + 32 * k, bh + ob + 32 * k, 1u);
+                    mma(d, D + AL + oa + 2 * k, D + BL + ob + 2 * k, k > 0);
+                    mma(d, D + oa + 2 * k, D + BL + ob + 2 * k, 1u);
+                    mma(d, D + AL + oa + 2 * k, D + BH + ob + 2 * k, 1u);
                 }
 #pragma unroll
                 for(int k = 0; k < 4; ++k)
-                    mma(d, base + oa + 32 * k, bh + ob + 32 * k, 1u);
+                    mma(d, D + oa + 2 * k, D + BH + ob + 2 * k, 1u);
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(gf_s32(&sh->mbar)) : "memory");
         }
