@@ -1137,7 +1137,8 @@ int ensureScratch(gf_engine *e) {
     return GF_OK;
 }
 
-// the mark of a word that no launch has written yet: a signalling NaN that no arithmetic result, status or zero equals
+// the mark of a word that no launch has written yet (one-launch rows, integrals): a signalling-NaN bit pattern, which no
+// arithmetic result (quiet NaNs only), status or zero equals
 static constexpr uint64_t kRowUnset = 0x7ff40000dead0001ull;
 
 // The integrals of toy e->int_toy from the entries that gf_ampng_sum wrote (the launch has ended, or the words are awaited:
@@ -1517,9 +1518,6 @@ struct NvtxScope {
     explicit NvtxScope(const char *name) { nvtxRangePushA(name); }
     ~NvtxScope() { nvtxRangePop(); }
 };
-
-// The host's mark of a one-launch row word not yet written: a signalling-NaN bit pattern, which no arithmetic
-// result (quiet NaNs only) and no status or zero the kernel stores can equal.
 
 // A row word written by the device into mapped host memory (one aligned 8-byte store), read as a double.
 static inline double wordValue(const uint64_t *p) {
