@@ -89,16 +89,17 @@ __device__ __forceinline__ void gf_tmem_st8(unsigned addr, const float *v) {
                  "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])) : "memory");
 }
 __device__ __forceinline__ void gf_tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-// One lane of a converged warp.  Issuing a tile's 16 or 32 MMAs is on the path of all its threads, which meet before and
+// One lane of a converged warp.  Issuing a tile's MMAs is on the path of all its threads, which meet before and
 // after it; from an elected lane it is shorter than from threadIdx.x == 0 (rebuild of 8 resonances 395 -> 379 us, of the
-// four-body model 928 -> 892 us).
+// four-body model 928 -> 892 us), and each 32-point block of a slice has its own warp issue its 16 MMAs, to its own
+// accumulator (four-body, two blocks: 892 -> 835 us).
 __device__ __forceinline__ bool gf_elect() {
     unsigned p;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
     return p != 0;
 }
 struct GfGramShared {
-    unsigned long long mbar, never; /* MMAs of a tile; a barrier that nothing arrives on (test of the failure path) */
+    unsigned long long mbar, never; /* MMAs of a tile (a commit per block); a barrier that nothing arrives on (test of the failure path) */
     unsigned tmem;
 };
 
@@ -132,7 +133,7 @@ struct GfGram {
         for(unsigned i = tid; i < (2 * ABYTES + (WT ? 2 * BBYTES : 0u)) / 16; i += 128) // padding rows stay zero
             reinterpret_cast<uint4 *>(ops)[i] = make_uint4(0u, 0u, 0u, 0u);
         if(tid == 0) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gf_s32(&sh->mbar)) : "memory");
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(gf_s32(&sh->mbar)), "r"(KB) : "memory");
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gf_s32(&sh->never)) : "memory");
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         }
@@ -238,23 +239,20 @@ struct GfGram {
         gf_tc_before();
         if(__syncthreads_or(!ok))
             return false;
-        if(threadIdx.x < 32 && gf_elect()) {
+        if(threadIdx.x < 32 * KB && gf_elect()) {
             gf_tc_after();
-            const unsigned D = desc();
+            const int b = KB == 1 ? 0 : (int)(threadIdx.x >> 5);
             constexpr unsigned AL = ABYTES >> 4, BH = WT ? 2 * AL : 0u, BL = WT ? BH + (BBYTES >> 4) : AL;
+            const unsigned oa = desc() + b * 1024u, ob = desc() + (WT ? b * N * 8u : b * 1024u), d = tmem + (unsigned)(b * N);
 #pragma unroll
-            for(int b = 0; b < KB; ++b) {
-                const unsigned oa = b * 1024u, ob = WT ? b * N * 8u : oa, d = tmem + (unsigned)(b * N);
-#pragma unroll
-                for(int k = 0; k < 4; ++k) { // 8 points: 32 bytes of every 128-byte row
-                    mma(d, D + AL + oa + 2 * k, D + BL + ob + 2 * k, k > 0);
-                    mma(d, D + oa + 2 * k, D + BL + ob + 2 * k, 1u);
-                    mma(d, D + AL + oa + 2 * k, D + BH + ob + 2 * k, 1u);
-                }
-#pragma unroll
-                for(int k = 0; k < 4; ++k)
-                    mma(d, D + oa + 2 * k, D + BH + ob + 2 * k, 1u);
+            for(int k = 0; k < 4; ++k) { // 8 points: 32 bytes of every 128-byte row
+                mma(d, oa + AL + 2 * k, ob + BL + 2 * k, k > 0);
+                mma(d, oa + 2 * k, ob + BL + 2 * k, 1u);
+                mma(d, oa + AL + 2 * k, ob + BH + 2 * k, 1u);
             }
+#pragma unroll
+            for(int k = 0; k < 4; ++k)
+                mma(d, oa + 2 * k, ob + BH + 2 * k, 1u);
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(gf_s32(&sh->mbar)) : "memory");
         }
         last = u;
